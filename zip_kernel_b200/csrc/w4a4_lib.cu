@@ -18,6 +18,7 @@
 #include "decode_gemm.cuh"
 #include "prefill_gemm.cuh"
 #include "prefill_pair_gemm.cuh"
+#include "prefill_wide_gemm.cuh"
 #include "peer_gather.cuh"
 
 namespace {
@@ -90,6 +91,8 @@ cudaError_t set_kernel_attributes() {
   set(pp::prefill_pair_gemm_kernel<true, false, false>, pp::smem_bytes(false));
   set(pp::prefill_pair_gemm_kernel<false, true, true>, pp::smem_bytes(true));
   set(pp::prefill_pair_gemm_kernel<true, true, true>, pp::smem_bytes(true));
+  set(wide::prefill_wide_gemm_kernel<false>, wide::smem_bytes());
+  set(wide::prefill_wide_gemm_kernel<true>, wide::smem_bytes());
   set(act_quant_kernel<128>, QUANT_MAX_SMEM);
   set(act_quant_kernel<QUANT_THREADS>, QUANT_MAX_SMEM);
   set(act_quant_kernel<128, SRC_RMSNORM>, QUANT_MAX_SMEM);
@@ -254,6 +257,7 @@ struct GemmArgs {
   bool do_dense;
   float sparse_weight;
   int xe_fmt;              // bytes of the expanded codes: W4A4_CODES_S8 / _E4M3 (prepared weights) / _E4M3_PACKED
+  bool widen;              // W4A4_CODES_E4M3 codes against packed weights, which the kernel widens itself
   void* ws;
   size_t ws_bytes;
   cudaStream_t stream;
@@ -402,6 +406,32 @@ bool f8_on_packed() {
   return e ? atoi(e) != 0 : false;
 }
 
+// CTA pairs with W4A4_PREFILL_PAIR=1 (see launch_prefill); read on every call, tests compare both in one process.
+bool pair_selected() {
+  const char* e = getenv("W4A4_PREFILL_PAIR");
+  return e && atoi(e) != 0;
+}
+
+// Tiles of 256 tokens (prefill_wide_gemm_kernel) or of 128 (prefill_gemm_kernel)?  Both run one CTA per SM, so a launch
+// takes waves x (K-steps x step + fixed) and the wide kernel wins unless its fewer tiles leave SMs idle.  Per
+// wave, us, fitted on B200 at 1.9 GHz (4096 -> 28672 and 14336 -> 4096, 512 to 8192 tokens): prepared weights
+// 0.60 n + 4.6 against 0.35 n + 5.8, packed weights 1.0 n + 4 against 0.55 n + 5.8.  Measured, both sides:
+// 14336 -> 4096, 512 tokens, prepared (64 or 128 tiles, one wave each) 117 against 69 us; 2944 -> 5000, 1537 tokens,
+// packed (2 against 4 waves) 70 against 83 us.
+bool wants_wide_tiles(int T, int K, int N, bool prepared, int sm_count) {
+  const long long rows = (N + 127) / 128;
+  const long long w256 = (rows * ((T + 255) / 256) + sm_count - 1) / sm_count, w128 = (rows * ((T + 127) / 128) + sm_count - 1) / sm_count;
+  const double n = K / 128;
+  return prepared ? w256 * (0.60 * n + 4.6) <= w128 * (0.35 * n + 5.8) : w256 * (1.0 * n + 4.0) <= w128 * (0.55 * n + 5.8);
+}
+
+// Code format of a tensor-core call on packed weights whose codes the library expands itself: e4m3 in natural
+// order for the wide kernel, s8 for the narrow one, unless one of the two selectable kernels is asked for.
+int packed_code_format(bool have_sums, int T, int K, int N, int sm_count) {
+  if (have_sums && f8_on_packed()) return W4A4_CODES_E4M3_PACKED;
+  return !pair_selected() && wants_wide_tiles(T, K, N, false, sm_count) ? W4A4_CODES_E4M3 : W4A4_CODES_S8;
+}
+
 // True when the call carries prepared weights for every operand it uses.
 bool has_prepared(const GemmArgs& a) {
   const bool has_sparse = a.nnz > 0 && a.sparse_weight != 0.f;
@@ -424,13 +454,15 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   // has an offset that only the sums can take out).
   const bool dump = a.acc_dump || a.acc_hi_dump;
   const bool has_sparse = a.nnz > 0 && a.sparse_weight != 0.f;
-  if (a.XE == nullptr)
-    a.xe_fmt = prep ? W4A4_CODES_E4M3
-                    : ((dump ? (a.flags & W4A4_FLAG_CODES_E4M3_PACKED) != 0 : (a.sum_X != nullptr && f8_on_packed()))
-                           ? W4A4_CODES_E4M3_PACKED : W4A4_CODES_S8);
+  if (a.XE == nullptr) {
+    a.xe_fmt = prep   ? W4A4_CODES_E4M3
+               : dump ? ((a.flags & W4A4_FLAG_CODES_E4M3_PACKED) ? W4A4_CODES_E4M3_PACKED : W4A4_CODES_S8)
+                      : packed_code_format(a.sum_X != nullptr, a.T, a.K, a.N, dev->sm_count);
+    a.widen = !prep && a.xe_fmt == W4A4_CODES_E4M3;
+  }
   if (prep && a.xe_fmt != W4A4_CODES_E4M3)
     return fail(W4A4_ERR_BAD_ARG, "prepared weights need activation codes expanded as W4A4_CODES_E4M3 (W4A4_FLAG_CODES_E4M3)");
-  if (!prep && a.xe_fmt == W4A4_CODES_E4M3)
+  if (!prep && !a.widen && a.xe_fmt == W4A4_CODES_E4M3)
     return fail(W4A4_ERR_BAD_ARG, "W4A4_CODES_E4M3 activation codes need prepared weights (w4a4_prepare_weights) for every "
                                   "operand in use; packed weights read W4A4_CODES_E4M3_PACKED or W4A4_CODES_S8");
   const bool f8 = a.xe_fmt != W4A4_CODES_S8;
@@ -440,6 +472,7 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   const int ng = a.K / BCOL;
   const int row_tiles = (a.N + pre::ROWS - 1) / pre::ROWS;
   const int tok_tiles = (a.T + pre::TN - 1) / pre::TN;
+  const bool wide_kernel = a.widen || (prep && !dump && !pair_selected() && wants_wide_tiles(a.T, a.K, a.N, true, dev->sm_count));
   if (tok_tiles > 65535) return fail(W4A4_ERR_UNSUPPORTED, "T=%d exceeds the grid limit of the tensor-core path", a.T);
   // expanded activations: given by the caller, or built here from the packed codes
   const void* XE = a.XE;
@@ -515,10 +548,14 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   // per tile (Llama-3-8B shapes, 2048 / 8192 tokens: packed 0.20 against 0.225 of the 8-bit tensor peak,
   // prepared 0.23 against 0.29): the step time is set by the fold warps' accumulator round trip, which the
   // pair leaves unchanged, and every hand-over now crosses two SMs.  Kept selectable for A/B runs.
-  const char* env_pair = getenv("W4A4_PREFILL_PAIR");
-  const bool pair = env_pair && atoi(env_pair) != 0 && pp::supported(a.T, a.K, a.N) && (!f8 || prep);
+  const bool pair = pair_selected() && pp::supported(a.T, a.K, a.N) && (!f8 || prep);
   cudaError_t e;
-  if (pair) {
+  if (wide_kernel) {
+    p.band = (p.band + 1) / 2;                  // tiles twice as wide
+    e = launch_ex(prep ? wide::prefill_wide_gemm_kernel<true> : wide::prefill_wide_gemm_kernel<false>,
+                  dim3(row_tiles, (a.T + wide::TN - 1) / wide::TN, 1), dim3(wide::THREADS), wide::smem_bytes(), a.stream, 1, tm_w,
+                  tm_wh, p);
+  } else if (pair) {
     const size_t smem = pp::smem_bytes(prep);
     void (*kern)(const CUtensorMap, const CUtensorMap, const pre::Params) =
         prep ? (dump ? pp::prefill_pair_gemm_kernel<true, true, true> : pp::prefill_pair_gemm_kernel<false, true, true>)
@@ -1101,7 +1138,8 @@ int w4a4_fused_quant_dense_sparse_prepared(const void* X, long long ldx, const i
   // the tensor-core kernel runs fp8 MMAs on e4m3 codes (natural order against prepared weights, even/odd
   // order against packed ones); the streaming kernel reads s8 codes
   a.xe_fmt = !tensor ? W4A4_CODES_S8
-             : has_prepared(a) ? W4A4_CODES_E4M3 : (f8_on_packed() ? W4A4_CODES_E4M3_PACKED : W4A4_CODES_S8);
+             : has_prepared(a) ? W4A4_CODES_E4M3 : packed_code_format(true, T, K, N, dev->sm_count);
+  a.widen = tensor && !has_prepared(a) && a.xe_fmt == W4A4_CODES_E4M3;
   rc = launch_quant(X, ldx, perm, nullptr, ws + wl.scale_x, nullptr, ws + wl.xe, reinterpret_cast<float*>(ws + wl.sumxf),
                     T, K, s, dev->sm_count, a.xe_fmt);
   if (rc) return rc;
