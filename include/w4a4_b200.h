@@ -103,6 +103,18 @@ int w4a4_silu_mul_quant(const void* GU, long long ldgu, const int32_t* perm, voi
  * that share one scratch buffer must be ordered on one stream. */
 size_t w4a4_workspace_bytes(int T, int K, int N, int nnz);
 
+/* The kernel that w4a4_fused_quant_dense_sparse (prepared = 0) or its _prepared form (prepared = 1: for every
+ * operand in use) runs on the current device for these sizes and flags, and the W4A4_CODES_* form it expands
+ * the activations to.  Host only, no counterpart in the reference.  A caller that expands activations itself
+ * gets the same output bits from W4A4_CODES_S8 wherever this reports W4A4_CODES_E4M3 without prepared weights:
+ * the *_expanded entry points read natural-order e4m3 codes against prepared weights only. */
+#define W4A4_KERNEL_STREAM    0   /* weight-streaming split-K kernel */
+#define W4A4_KERNEL_TILES_128 1   /* tensor-core kernel, 128-token tiles */
+#define W4A4_KERNEL_TILES_256 2   /* tensor-core kernel, 256-token tiles */
+#define W4A4_KERNEL_PAIRS     3   /* tensor-core kernel on CTA pairs (W4A4_PREFILL_PAIR=1) */
+int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared, int* kernel /* host */,
+                     int* code_format /* host */);
+
 /* Replaces fused_dense_sparse_mma_int4_launch, fused_gemv_decode_launch and
  * fused_gemv_smallT_launch (bindings.cc:187-235; kernels
  * fused_dense_sparse_mma_int4.cu:184-1190, fused_gemv_decode.cu:54-191,
@@ -226,9 +238,10 @@ int w4a4_fused_quant_dense_sparse_prepared(const void* X, long long ldx, const i
  * prepared weights for every operand in use, both flags at once.  A call with e4m3 codes of either form
  * always runs the tensor-core kernel, whatever the token count (the streaming kernel reads s8 codes;
  * W4A4_FLAG_FORCE_STREAM with e4m3 codes is W4A4_ERR_BAD_ARG).  The entry points that expand the codes
- * themselves pick W4A4_CODES_E4M3 when prepared weights are given, else W4A4_CODES_S8 - or
- * W4A4_CODES_E4M3_PACKED when the environment variable W4A4_PREFILL_F8=1 is set and the call carries
- * the group sums. */
+ * themselves pick the form their kernel reads (w4a4_gemm_choice): W4A4_CODES_S8 for the streaming kernel and
+ * for 128-token tiles on packed weights, W4A4_CODES_E4M3 for prepared weights and for 256-token tiles, which
+ * widen packed weights to e4m3 themselves - or W4A4_CODES_E4M3_PACKED when the environment variable
+ * W4A4_PREFILL_F8=1 is set, the weights are packed and the call carries the group sums. */
 #define W4A4_CODES_S8   0
 #define W4A4_CODES_E4M3 1
 #define W4A4_CODES_E4M3_PACKED 2

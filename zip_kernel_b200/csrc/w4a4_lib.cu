@@ -256,7 +256,7 @@ struct GemmArgs {
   int T, K, N, nnz, flags;
   bool do_dense;
   float sparse_weight;
-  int xe_fmt;              // bytes of the expanded codes: W4A4_CODES_S8 / _E4M3 (prepared weights) / _E4M3_PACKED
+  int xe_fmt;              // bytes of the expanded codes: W4A4_CODES_*
   bool widen;              // W4A4_CODES_E4M3 codes against packed weights, which the kernel widens itself
   void* ws;
   size_t ws_bytes;
@@ -425,11 +425,20 @@ bool wants_wide_tiles(int T, int K, int N, bool prepared, int sm_count) {
   return prepared ? w256 * (0.60 * n + 4.6) <= w128 * (0.35 * n + 5.8) : w256 * (1.0 * n + 4.0) <= w128 * (0.55 * n + 5.8);
 }
 
-// Code format of a tensor-core call on packed weights whose codes the library expands itself: e4m3 in natural
-// order for the wide kernel, s8 for the narrow one, unless one of the two selectable kernels is asked for.
-int packed_code_format(bool have_sums, int T, int K, int N, int sm_count) {
-  if (have_sums && f8_on_packed()) return W4A4_CODES_E4M3_PACKED;
-  return !pair_selected() && wants_wide_tiles(T, K, N, false, sm_count) ? W4A4_CODES_E4M3 : W4A4_CODES_S8;
+struct GemmChoice {
+  int kernel;              // W4A4_KERNEL_*
+  int codes;               // W4A4_CODES_* that kernel reads
+};
+
+// The tensor-core kernel of a call whose codes the library expands itself, and the form it expands them to.  Prepared
+// weights: natural-order e4m3 codes.  Packed weights: the wide kernel widens them to e4m3 itself and reads
+// natural-order codes too, the narrow one widens them to s8; W4A4_PREFILL_F8=1 and W4A4_PREFILL_PAIR=1 go first.
+GemmChoice choose_tensor_kernel(int T, int K, int N, bool prepared, bool have_sums, int sm_count) {
+  if (!prepared && have_sums && f8_on_packed()) return {W4A4_KERNEL_TILES_128, W4A4_CODES_E4M3_PACKED};
+  const int narrow_codes = prepared ? W4A4_CODES_E4M3 : W4A4_CODES_S8;
+  if (pair_selected()) return {w4a4::pp::supported(T, K, N) ? W4A4_KERNEL_PAIRS : W4A4_KERNEL_TILES_128, narrow_codes};
+  if (wants_wide_tiles(T, K, N, prepared, sm_count)) return {W4A4_KERNEL_TILES_256, W4A4_CODES_E4M3};
+  return {W4A4_KERNEL_TILES_128, narrow_codes};
 }
 
 // True when the call carries prepared weights for every operand it uses.
@@ -447,17 +456,16 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   GemmArgs a = a_in;
   const bool prep = has_prepared(a);
   // The expanded codes say which instantiation runs: e4m3 in natural order goes with prepared weights (fp8
-  // MMAs on bytes as they land), e4m3 in even/odd order with packed weights read as e4m3 numbers (fp8
-  // MMAs, see nib_lo_off8), s8 with packed weights widened to s8 (integer MMAs).  When the library expands
-  // the codes itself it picks the e4m3 form that matches the weights; the integer instantiation remains for
-  // callers' s8 codes and for calls that carry no activation group sums (the e4m3 form of packed weights
-  // has an offset that only the sums can take out).
+  // MMAs on bytes as they land) or with packed weights that the wide kernel widens to e4m3 (`widen`: only where
+  // the library expands the codes itself), e4m3 in even/odd order with packed weights read as e4m3 numbers (fp8
+  // MMAs, see nib_lo_off8; needs the group sums, which alone can take its offset out), s8 with packed weights
+  // widened to s8 (integer MMAs).  When the library expands the codes itself choose_tensor_kernel picks.
   const bool dump = a.acc_dump || a.acc_hi_dump;
   const bool has_sparse = a.nnz > 0 && a.sparse_weight != 0.f;
   if (a.XE == nullptr) {
     a.xe_fmt = prep   ? W4A4_CODES_E4M3
                : dump ? ((a.flags & W4A4_FLAG_CODES_E4M3_PACKED) ? W4A4_CODES_E4M3_PACKED : W4A4_CODES_S8)
-                      : packed_code_format(a.sum_X != nullptr, a.T, a.K, a.N, dev->sm_count);
+                      : choose_tensor_kernel(a.T, a.K, a.N, false, a.sum_X != nullptr, dev->sm_count).codes;
     a.widen = !prep && a.xe_fmt == W4A4_CODES_E4M3;
   }
   if (prep && a.xe_fmt != W4A4_CODES_E4M3)
@@ -472,7 +480,8 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   const int ng = a.K / BCOL;
   const int row_tiles = (a.N + pre::ROWS - 1) / pre::ROWS;
   const int tok_tiles = (a.T + pre::TN - 1) / pre::TN;
-  const bool wide_kernel = a.widen || (prep && !dump && !pair_selected() && wants_wide_tiles(a.T, a.K, a.N, true, dev->sm_count));
+  const bool wide_kernel =
+      a.widen || (prep && !dump && choose_tensor_kernel(a.T, a.K, a.N, true, true, dev->sm_count).kernel == W4A4_KERNEL_TILES_256);
   if (tok_tiles > 65535) return fail(W4A4_ERR_UNSUPPORTED, "T=%d exceeds the grid limit of the tensor-core path", a.T);
   // expanded activations: given by the caller, or built here from the packed codes
   const void* XE = a.XE;
@@ -924,6 +933,22 @@ size_t w4a4_workspace_bytes(int T, int K, int N, int nnz) {
   return ws_layout(T, K).total;
 }
 
+int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared, int* kernel, int* code_format) {
+  begin_call();
+  int rc = check_common(T, K, N, nnz);
+  if (rc) return rc;
+  CHECK_ARG(kernel && code_format, "NULL output pointer");
+  DeviceInfo* dev = nullptr;
+  rc = current_device(&dev);
+  if (rc) return rc;
+  const GemmChoice c = wants_tensor_path(T, K, N, flags, dev->sm_count, prepared != 0)
+                           ? choose_tensor_kernel(T, K, N, prepared != 0, true, dev->sm_count)
+                           : GemmChoice{W4A4_KERNEL_STREAM, W4A4_CODES_S8};
+  *kernel = c.kernel;
+  *code_format = c.codes;
+  return W4A4_OK;
+}
+
 int w4a4_fused_dense_sparse(const void* W_low, const void* W_high, const int32_t* hp_row_offsets,
                             const int32_t* hp_col_indices, const void* X_s4, const void* scale_u4,
                             const void* zero_u4, const int32_t* sum_X, const void* scale_x, void* Y, int T, int K,
@@ -1135,10 +1160,8 @@ int w4a4_fused_quant_dense_sparse_prepared(const void* X, long long ldx, const i
   a.W_low_prep = W_low_prepared; a.W_high_prep = W_high_prepared;
   const bool tensor = wants_tensor_path(T, K, N, flags, dev->sm_count, has_prepared(a));
   if (!tensor || !has_prepared(a)) a.W_low_prep = a.W_high_prep = nullptr;
-  // the tensor-core kernel runs fp8 MMAs on e4m3 codes (natural order against prepared weights, even/odd
-  // order against packed ones); the streaming kernel reads s8 codes
-  a.xe_fmt = !tensor ? W4A4_CODES_S8
-             : has_prepared(a) ? W4A4_CODES_E4M3 : packed_code_format(true, T, K, N, dev->sm_count);
+  // what the chosen tensor-core kernel reads; the streaming kernel reads s8 codes
+  a.xe_fmt = tensor ? choose_tensor_kernel(T, K, N, has_prepared(a), true, dev->sm_count).codes : W4A4_CODES_S8;
   a.widen = tensor && !has_prepared(a) && a.xe_fmt == W4A4_CODES_E4M3;
   rc = launch_quant(X, ldx, perm, nullptr, ws + wl.scale_x, nullptr, ws + wl.xe, reinterpret_cast<float*>(ws + wl.sumxf),
                     T, K, s, dev->sm_count, a.xe_fmt);

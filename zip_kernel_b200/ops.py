@@ -13,6 +13,7 @@ Differences that follow from the B200 design (results are unaffected):
 
 from __future__ import annotations
 
+import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -115,6 +116,16 @@ def _code_format(e4m3) -> int:
 
 def _code_flag(e4m3) -> int:
     return (0, _lib.FLAG_CODES_E4M3, _lib.FLAG_CODES_E4M3_PACKED)[_code_format(e4m3)]
+
+
+def gemm_choice(T: int, d_out: int, d_in: int, n_hp_blocks: int = 0, *, prepared: bool = False,
+                force: Optional[str] = None, device=None) -> Tuple[int, int]:
+    """``(kernel, code format)`` (``_lib.KERNEL_*``, ``_lib.CODES_*``) of a fused call with these sizes on ``device``."""
+    kernel, codes = ctypes.c_int(0), ctypes.c_int(0)
+    with _lib.on_device(torch.device("cuda") if device is None else device):
+        _lib.check(_L.w4a4_gemm_choice(int(T), int(d_in), int(d_out), int(n_hp_blocks), _flags(False, force), int(prepared),
+                                       ctypes.byref(kernel), ctypes.byref(codes)), "gemm_choice")
+    return kernel.value, codes.value
 
 
 def _fused_prologue(which: str, X2: torch.Tensor, K: int, perm, norm_weight, eps: float, expanded: bool, e4m3):
@@ -586,4 +597,5 @@ __all__ = [
     "rmsnorm_quant_cuda",
     "silu_mul_quant_cuda",
     "perm_or_none",
+    "gemm_choice",
 ]

@@ -17,7 +17,7 @@ import os
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from .pack_utils import BCOL, V9WeightContainer, unpack_s4_le
 
 DECODE_T_THRESHOLD = 128
@@ -80,11 +80,16 @@ def _gemm_on_expanded(quantised, W: V9WeightContainer, lead_shape, e4m3) -> torc
 
 
 def _wants_e4m3(W: V9WeightContainer, T: int):
-    # the many-token kernel runs fp8 MMAs: on the prepared copy when the container has one, else on the packed
-    # arrays; below its threshold the packed arrays are streamed against s8 codes
-    if T < 256:
+    # The codes v9_linear_forward would use for this many tokens, so that both round alike.  Where it runs wide tiles
+    # on packed weights (natural-order e4m3 codes that only a prepared copy can be read against here), s8 codes
+    # and narrow tiles give the same bits.
+    if T < 64:                                       # always streamed against s8 codes
         return False
-    return True if W.prepared is not None else "packed"
+    codes = ops.gemm_choice(T, W.d_out, W.d_in, W.n_hp_blocks, prepared=W.prepared is not None,
+                            device=W.W_low_packed.device)[1]
+    if codes == _lib.CODES_E4M3_PACKED:
+        return "packed"
+    return codes == _lib.CODES_E4M3 and W.prepared is not None
 
 
 def v9_linear_forward_rmsnorm(X_fp16: torch.Tensor, norm_weight: torch.Tensor, eps: float,
