@@ -70,6 +70,9 @@ int w4a4_device_error(int* word /* host */, void* stream);
  * w4a4_device_error then returns W4A4_ERR_DEVICE with word = 0x40000000 | (0x7e << 8), and the
  * context stays usable. */
 int w4a4_selftest_bounded_wait(int polls, void* stream);
+/* The same with the wait of the 256-token kernel, whose polls may sleep in hardware: it gives up after one to a few
+ * seconds, never earlier. */
+int w4a4_selftest_suspended_wait(void* stream);
 
 /* Replaces activation_quant_launch (bindings.cc:113-122; kernel
  * cuda_kernel/csrc/activation_quant/activation_quant.cu:699-865).

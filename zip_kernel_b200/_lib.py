@@ -30,6 +30,7 @@ SIGNATURES = {
     "w4a4_last_error": (_c.c_char_p, []),
     "w4a4_device_error": (_INT, [_c.POINTER(_INT), _PTR]),
     "w4a4_selftest_bounded_wait": (_INT, [_INT, _PTR]),
+    "w4a4_selftest_suspended_wait": (_INT, [_PTR]),
     "w4a4_activation_quant": (_INT, [_PTR, _LL, _PTR, _PTR, _PTR, _PTR, _INT, _INT, _PTR]),
     "w4a4_rmsnorm_quant": (_INT, [_PTR, _LL, _PTR, _c.c_float] + [_PTR] * 6 + [_INT, _INT, _INT, _PTR]),
     "w4a4_silu_mul_quant": (_INT, [_PTR, _LL] + [_PTR] * 6 + [_INT, _INT, _INT, _PTR]),

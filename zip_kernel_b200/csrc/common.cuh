@@ -12,9 +12,11 @@ constexpr int BROW = 128;   // residual block rows  (reference: csrc/common/arch
 constexpr int BCOL = 128;   // quantisation group / residual block columns (arch.cuh:31)
 constexpr int GROUP_BYTES = BCOL / 2;   // packed bytes of one group of one row
 
-// Every device-side wait polls at most this many times, then records an error
-// and gives up, so a logic error can never leave the GPU spinning.  (A long
-// hardware suspend hint on try_wait was measured slower than plain polling:
+// Every wait through the functions below polls at most this many times, then records
+// an error and gives up, so a logic error can never leave the GPU spinning.  (A poll
+// that misses lasts about 4 us on B200 whatever the hint, so this is about 17 s.  The
+// 256-token tensor-core kernel has a wait of its own, bounded in time.  In the streaming
+// kernel a hardware suspend hint on try_wait was measured slower than plain polling:
 // the wake-up adds latency to every pipeline step.)
 constexpr uint32_t WAIT_POLL_LIMIT = 1u << 22;
 

@@ -92,17 +92,31 @@ __device__ __forceinline__ void umma_tf32(uint32_t d, uint64_t a, uint64_t b, ui
       : "memory");
 }
 
-// Bounded wait whose polls may sleep in hardware (up to 20 us each, about a second in all): the roles of this kernel
-// wait for hundreds of clocks at a time, and polling takes issue slots and instruction fetches from the fold
-// warps of the same scheduler (-2 % time against plain polling).
+// Bounded wait whose polls may sleep in hardware (up to 20 us each): the roles of this kernel wait for hundreds of
+// clocks at a time, and polling takes issue slots and instruction fetches from the fold warps of the same
+// scheduler (-2 % time against plain polling).  The hint bounds a poll from above only - a poll that misses returns
+// after about 4 us on B200 - so the count of polls alone (65536: 0.26 s) does not say how long the wait lasts: it
+// gives up after WAIT_POLLS polls AND WAIT_NS nanoseconds (a count too, because the timer also runs while another
+// process has the GPU).
+constexpr uint32_t WAIT_POLLS = 1u << 16;
+constexpr uint64_t WAIT_NS = 1000000000;
+__device__ __forceinline__ uint64_t timer_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ bool try_wait_suspend(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(20000) : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ bool wait_suspend(uint64_t* bar, uint32_t parity, int site) {
-  for (uint32_t i = 0; i < (1u << 16); ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(20000) : "memory");
-    if (ok) return true;
-  }
+  if (try_wait_suspend(bar, parity)) return true;
+  const uint64_t t0 = timer_ns();
+  for (uint32_t i = 0; i < WAIT_POLLS || timer_ns() - t0 < WAIT_NS; ++i)
+    if (try_wait_suspend(bar, parity)) return true;
   record_error(site, parity);
   return false;
 }
@@ -175,6 +189,9 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       int s = 0;
       uint32_t ph = 1;
       for (int n = 0; n < n_steps; ++n) {
+        // From here on this role waits for MMAs, and they for the preceding kernel's output: that time is not
+        // this kernel's, so no bounded wait runs during it (here and in the roles below).
+        if (n == STAGES) grid_dependency_wait();
         if (n >= STAGES && !wait_suspend(&done[s], ph, SITE_WIDE_W)) break;
         uint64_t* bar = PREP ? &ready[s] : &w_full[s];
         TRACE(0, n);
@@ -217,6 +234,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       int s = par, buf = par;
       uint32_t ph = 0;
       bool ok = true;
+      grid_dependency_wait();
       for (int n = par; n < n_steps; n += 2) {
         ok = wait_suspend(&ready[s], ph, SITE_WIDE_READY);
         if (!ok) break;
@@ -285,6 +303,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       }
     };
     auto store_tab = [&](int k, const float (&f)[TAB]) {
+      if (PREP && k == 2) grid_dependency_wait();          // packed weights: after the step STAGES, below
       if (ok && k >= 2) ok = __all_sync(0xffffffffu, wait_suspend(&tab_empty[k & 1], ((k >> 1) - 1) & 1, SITE_WIDE_TAB));
       if (!ok) return;
 #pragma unroll
@@ -307,6 +326,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
           store_tab(n / TAB, f);
           if (n / TAB + 1 < n_tab) load_tab(n / TAB + 1, f);
         }
+        if (n == STAGES) grid_dependency_wait();           // the first STAGES weight copies depend on nothing
         if (ok) ok = __all_sync(0xffffffffu, wait_suspend(&w_full[s], ph, SITE_WIDE_PACKED));
         const uint32_t slot = ring_a + s * SLOT;
         // the row's 64 packed bytes: 16-byte chunks stored at chunk ^ ((row >> 1) & 3) by the 64-byte swizzle

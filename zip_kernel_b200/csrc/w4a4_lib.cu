@@ -731,6 +731,16 @@ __global__ void selftest_wait_kernel(uint32_t polls) {
   }
 }
 
+// The same for the wait whose polls sleep in hardware (256-token tiles); lasts WAIT_NS or a little longer.
+__global__ void selftest_suspended_wait_kernel() {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    w4a4::mbar_init(&bar, 1);
+    w4a4::mbar_fence_init();
+    w4a4::wide::wait_suspend(&bar, 0, SITE_SELFTEST);
+  }
+}
+
 #ifdef W4A4_TRACE
 long long* trace_ptr() { return g_trace_ptr; }
 #endif
@@ -779,6 +789,14 @@ int w4a4_selftest_bounded_wait(int polls, void* stream) {
   begin_call();
   CHECK_ARG(polls >= 1 && polls <= (1 << 20), "polls must be in 1..2^20, got %d", polls);
   selftest_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>((uint32_t)polls);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(W4A4_ERR_LAUNCH, "self-test kernel launch: %s", cudaGetErrorString(e));
+  return W4A4_OK;
+}
+
+int w4a4_selftest_suspended_wait(void* stream) {
+  begin_call();
+  selftest_suspended_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(W4A4_ERR_LAUNCH, "self-test kernel launch: %s", cudaGetErrorString(e));
   return W4A4_OK;
