@@ -69,7 +69,7 @@ struct Layout {
 };
 inline size_t smem_bytes() { return 1024 + Layout::total; }
 
-enum : int { SITE_WIDE_W = 48, SITE_WIDE_X, SITE_WIDE_READY, SITE_WIDE_PACKED, SITE_WIDE_TAB, SITE_WIDE_Z, SITE_WIDE_ACC };
+enum : int { SITE_WIDE_W = 72, SITE_WIDE_X, SITE_WIDE_READY, SITE_WIDE_PACKED, SITE_WIDE_TAB, SITE_WIDE_Z, SITE_WIDE_ACC };
 
 __device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
