@@ -181,6 +181,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
   const int n_steps = p.nd + (b_hi - b_lo);
   // ring entries 0 .. n_steps - 1 are K-steps, n_steps .. n_steps + n_z - 1 the zero-point products
   const int n_z = p.sumxf != nullptr ? (p.nd + TAB - 1) / TAB : 0;
+  bool ok = true;                                 // no wait of this thread has given up
 
   if (warp < WARP_HELP0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_ISSUE));
@@ -192,7 +193,8 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         // From here on this role waits for MMAs, and they for the preceding kernel's output: that time is not
         // this kernel's, so no bounded wait runs during it (here and in the roles below).
         if (n == STAGES) grid_dependency_wait();
-        if (n >= STAGES && !wait_suspend(&done[s], ph, SITE_WIDE_W)) break;
+        if (n >= STAGES) ok = wait_suspend(&done[s], ph, SITE_WIDE_W);
+        if (!ok) break;
         uint64_t* bar = PREP ? &ready[s] : &w_full[s];
         TRACE(0, n);
         mbar_arrive_expect_tx(bar, PREP ? W_BYTES : W_BYTES / 2);
@@ -208,7 +210,6 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       const uint32_t bytes = (uint32_t)n_mma * BCOL;     // rows up to the 16-token padding: inside the buffer
       int s = 0;
       uint32_t ph = 1;
-      bool ok = true;
       for (int n = 0; n < n_steps; ++n) {
         const int g = n < p.nd ? n : ld_plain(p.hp_col_indices + b_lo + n - p.nd);
         if (n >= STAGES) ok = wait_suspend(&done[s], ph, SITE_WIDE_X);
@@ -233,7 +234,6 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       const uint64_t a0 = pre::smem_desc_sw128(sm), b0 = pre::smem_desc_sw128(sm + W_BYTES);
       int s = par, buf = par;
       uint32_t ph = 0;
-      bool ok = true;
       grid_dependency_wait();
       for (int n = par; n < n_steps; n += 2) {
         ok = wait_suspend(&ready[s], ph, SITE_WIDE_READY);
@@ -255,7 +255,8 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       if (ok && (n_steps & 1) == par) {
         const uint32_t d = tmem_base + buf * TN;
         for (int k = 0; k < n_z; ++k) {
-          if (!wait_suspend(&ready[s], ph, SITE_WIDE_Z)) break;
+          ok = wait_suspend(&ready[s], ph, SITE_WIDE_Z);
+          if (!ok) break;
           pre::tc_fence_after();
           const uint64_t off = (uint64_t)(s * (SLOT >> 4));
 #pragma unroll
@@ -275,7 +276,6 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     const int n_tab = (n_steps + TAB - 1) / TAB;
     const __half* srow = p.scale_u4 + (size_t)min(row, p.N - 1) * p.ng;
     const bool row_live = row < p.N;
-    bool ok = true;
     // scale factors of the 16 steps of table k: dense groups in order, then the residual blocks' groups
     auto load_tab = [&](int k, float (&f)[TAB]) {
 #pragma unroll
@@ -424,7 +424,6 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     float y[COLS];
 #pragma unroll
     for (int i = 0; i < COLS; ++i) y[i] = 0.f;
-    bool ok = true;
     // the accumulators start out free
     if (lane == 0)
       for (int i = 0; i < ACC_BUFS && i <= last_q; ++i) mbar_arrive(&ready[i]);
@@ -532,9 +531,15 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
 #ifdef W4A4_TRACE
   if (tid == WARP_FOLD0 * 32) { TRACE(8, 0); if (lin == p.trace_cta) p.trace[8 * 64 + 1] = t_start; }
 #endif
-  // common exit: every role falls through to here, then the allocating warp frees tensor memory
+  // Common exit: every role falls through to here, then the allocating warp frees tensor memory.  After a wait that
+  // gave up copies and MMAs may still be in flight, on barriers that also count arrivals which will not come: the
+  // block then stays for a millisecond, many times what they need, before its memory is handed on.
   pre::tc_fence_before();
-  __syncthreads();
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0)
+      for (const uint64_t t0 = timer_ns(); timer_ns() - t0 < 1000000;) __nanosleep(1000);
+    __syncthreads();
+  }
   if (warp == WARP_MMA) {
     pre::tc_fence_after();
     pre::tmem_dealloc(tmem_base, pre::TMEM_COLS);
