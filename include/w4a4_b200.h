@@ -55,6 +55,9 @@ enum {
 #define W4A4_FLAG_CODES_E4M3      0x8  /* *_expanded entry points: XE holds W4A4_CODES_E4M3 bytes (for prepared weights) */
 #define W4A4_FLAG_CODES_E4M3_PACKED 0x10 /* *_expanded entry points: XE holds W4A4_CODES_E4M3_PACKED bytes (for packed
                                             weights); w4a4_dump_accumulators: run the fp8 instantiation on packed weights */
+#define W4A4_FLAG_TILES_128       0x20 /* where the tensor-core kernel runs: 128-token tiles      */
+#define W4A4_FLAG_TILES_256       0x40 /* ... 256-token tiles (same output bits); W4A4_ERR_BAD_ARG with caller-expanded codes
+                                            other than W4A4_CODES_E4M3 and for w4a4_dump_accumulators          */
 
 int w4a4_abi_version(void);
 const char* w4a4_status_string(int status);

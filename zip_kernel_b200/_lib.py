@@ -67,6 +67,8 @@ FLAG_FORCE_STREAM = 0x2
 FLAG_FORCE_TENSOR = 0x4
 FLAG_CODES_E4M3 = 0x8
 FLAG_CODES_E4M3_PACKED = 0x10
+FLAG_TILES_128 = 0x20
+FLAG_TILES_256 = 0x40
 CODES_S8, CODES_E4M3, CODES_E4M3_PACKED = 0, 1, 2
 KERNEL_STREAM, KERNEL_TILES_128, KERNEL_TILES_256, KERNEL_PAIRS = 0, 1, 2, 3
 

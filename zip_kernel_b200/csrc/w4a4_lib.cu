@@ -412,17 +412,30 @@ bool pair_selected() {
   return e && atoi(e) != 0;
 }
 
+// Sizes that a choice of kernel goes by: `dense` groups of K in every block-row, `nnz` residual blocks over all.
+struct GemmSizes {
+  int T, K, N;
+  bool dense;
+  int nnz;
+};
+
 // Tiles of 256 tokens (prefill_wide_gemm_kernel) or of 128 (prefill_gemm_kernel)?  Both run one CTA per SM, so a launch
-// takes waves x (K-steps x step + fixed) and the wide kernel wins unless its fewer tiles leave SMs idle.  Per
-// wave, us, fitted on B200 at 1.9 GHz (4096 -> 28672 and 14336 -> 4096, 512 to 8192 tokens): prepared weights
-// 0.60 n + 4.6 against 0.35 n + 5.8, packed weights 1.0 n + 4 against 0.55 n + 5.8.  Measured, both sides:
-// 14336 -> 4096, 512 tokens, prepared (64 or 128 tiles, one wave each) 117 against 69 us; 2944 -> 5000, 1537 tokens,
-// packed (2 against 4 waves) 70 against 83 us.
-bool wants_wide_tiles(int T, int K, int N, bool prepared, int sm_count) {
-  const long long rows = (N + 127) / 128;
-  const long long w256 = (rows * ((T + 255) / 256) + sm_count - 1) / sm_count, w128 = (rows * ((T + 127) / 128) + sm_count - 1) / sm_count;
-  const double n = K / 128;
-  return prepared ? w256 * (0.60 * n + 4.6) <= w128 * (0.35 * n + 5.8) : w256 * (1.0 * n + 4.0) <= w128 * (0.55 * n + 5.8);
+// takes waves x (K-steps x step + fixed), the steps counted with the residual blocks.  The constants (us) were
+// fitted on B200 at 1.9 GHz to the measured winner of 254 launches whose waves differ (d_in 128 to 14336, d_out
+// 1024 to 28672, 64 to 2048 tokens, 0 / 5 / 15 % residual blocks, residual-only calls): none of them loses more
+// than 1 %.  Near the line: 14336 -> 4096, 600 tokens, prepared (1 against 2 waves) 109 against 113 us; 14336 -> 28672,
+// 512 tokens, prepared (4 against 7) 380 against 355 us; 4096 -> 6144, 1024 tokens, packed (2 against 3) 83 against 81.
+// With equally many waves the narrow tile's shorter steps win (14336 -> 4096, 512 tokens, prepared 105 against 64 us; 256 ->
+// 6144, 384 tokens, packed 12.6 against 10.7; 15 % blocks of 4096 -> 4096 alone, 512 tokens 18.2 against 15.5), except
+// where a few steps of few tokens leave mostly the fixed part (512 -> 4096, 128 tokens, packed 10.7 against 11.4
+// us; 256 -> 4096, 192 tokens, prepared 8.5 against 9.0).
+bool wants_wide_tiles(const GemmSizes& z, bool prepared, int sm_count) {
+  const long long rows = (z.N + 127) / 128;
+  const long long w256 = (rows * ((z.T + 255) / 256) + sm_count - 1) / sm_count;
+  const long long w128 = (rows * ((z.T + 127) / 128) + sm_count - 1) / sm_count;
+  if (w256 == w128) return z.dense && ((z.T <= 128 && z.K <= 512) || (prepared && z.T <= 256 && z.K <= 256));
+  const double n = (z.dense ? z.K / 128 : 0) + (double)z.nnz / (double)rows;
+  return prepared ? w256 * (0.72 * n + 3.0) <= w128 * (0.37 * n + 6.5) : w256 * (0.94 * n + 3.5) <= w128 * (0.55 * n + 4.5);
 }
 
 struct GemmChoice {
@@ -432,13 +445,22 @@ struct GemmChoice {
 
 // The tensor-core kernel of a call whose codes the library expands itself, and the form it expands them to.  Prepared
 // weights: natural-order e4m3 codes.  Packed weights: the wide kernel widens them to e4m3 itself and reads
-// natural-order codes too, the narrow one widens them to s8; W4A4_PREFILL_F8=1 and W4A4_PREFILL_PAIR=1 go first.
-GemmChoice choose_tensor_kernel(int T, int K, int N, bool prepared, bool have_sums, int sm_count) {
-  if (!prepared && have_sums && f8_on_packed()) return {W4A4_KERNEL_TILES_128, W4A4_CODES_E4M3_PACKED};
+// natural-order codes too, the narrow one widens them to s8.  The tile a caller's flag asks for goes first, then
+// W4A4_PREFILL_F8=1 and W4A4_PREFILL_PAIR=1, then the rule.
+GemmChoice choose_tensor_kernel(const GemmSizes& z, int flags, bool prepared, bool have_sums, int sm_count) {
+  if (flags & W4A4_FLAG_TILES_256) return {W4A4_KERNEL_TILES_256, W4A4_CODES_E4M3};
   const int narrow_codes = prepared ? W4A4_CODES_E4M3 : W4A4_CODES_S8;
-  if (pair_selected()) return {w4a4::pp::supported(T, K, N) ? W4A4_KERNEL_PAIRS : W4A4_KERNEL_TILES_128, narrow_codes};
-  if (wants_wide_tiles(T, K, N, prepared, sm_count)) return {W4A4_KERNEL_TILES_256, W4A4_CODES_E4M3};
+  if (flags & W4A4_FLAG_TILES_128) return {W4A4_KERNEL_TILES_128, narrow_codes};
+  if (!prepared && have_sums && f8_on_packed()) return {W4A4_KERNEL_TILES_128, W4A4_CODES_E4M3_PACKED};
+  if (pair_selected()) return {w4a4::pp::supported(z.T, z.K, z.N) ? W4A4_KERNEL_PAIRS : W4A4_KERNEL_TILES_128, narrow_codes};
+  if (wants_wide_tiles(z, prepared, sm_count)) return {W4A4_KERNEL_TILES_256, W4A4_CODES_E4M3};
   return {W4A4_KERNEL_TILES_128, narrow_codes};
+}
+
+int check_tile_flags(int flags) {
+  CHECK_ARG((flags & W4A4_FLAG_TILES_128) == 0 || (flags & W4A4_FLAG_TILES_256) == 0,
+            "W4A4_FLAG_TILES_128 and W4A4_FLAG_TILES_256 exclude each other");
+  return W4A4_OK;
 }
 
 // True when the call carries prepared weights for every operand it uses.
@@ -462,10 +484,11 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   // widened to s8 (integer MMAs).  When the library expands the codes itself choose_tensor_kernel picks.
   const bool dump = a.acc_dump || a.acc_hi_dump;
   const bool has_sparse = a.nnz > 0 && a.sparse_weight != 0.f;
+  const GemmSizes sizes{a.T, a.K, a.N, a.do_dense, has_sparse ? a.nnz : 0};
   if (a.XE == nullptr) {
     a.xe_fmt = prep   ? W4A4_CODES_E4M3
                : dump ? ((a.flags & W4A4_FLAG_CODES_E4M3_PACKED) ? W4A4_CODES_E4M3_PACKED : W4A4_CODES_S8)
-                      : choose_tensor_kernel(a.T, a.K, a.N, false, a.sum_X != nullptr, dev->sm_count).codes;
+                      : choose_tensor_kernel(sizes, a.flags, false, a.sum_X != nullptr, dev->sm_count).codes;
     a.widen = !prep && a.xe_fmt == W4A4_CODES_E4M3;
   }
   if (prep && a.xe_fmt != W4A4_CODES_E4M3)
@@ -481,7 +504,9 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   const int row_tiles = (a.N + pre::ROWS - 1) / pre::ROWS;
   const int tok_tiles = (a.T + pre::TN - 1) / pre::TN;
   const bool wide_kernel =
-      a.widen || (prep && !dump && choose_tensor_kernel(a.T, a.K, a.N, true, true, dev->sm_count).kernel == W4A4_KERNEL_TILES_256);
+      a.widen || (prep && !dump && choose_tensor_kernel(sizes, a.flags, true, true, dev->sm_count).kernel == W4A4_KERNEL_TILES_256);
+  if ((a.flags & W4A4_FLAG_TILES_256) && !wide_kernel)
+    return fail(W4A4_ERR_BAD_ARG, "256-token tiles read neither W4A4_CODES_S8 nor W4A4_CODES_E4M3_PACKED codes and dump no accumulators");
   if (tok_tiles > 65535) return fail(W4A4_ERR_UNSUPPORTED, "T=%d exceeds the grid limit of the tensor-core path", a.T);
   // expanded activations: given by the caller, or built here from the packed codes
   const void* XE = a.XE;
@@ -557,7 +582,7 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   // per tile (Llama-3-8B shapes, 2048 / 8192 tokens: packed 0.20 against 0.225 of the 8-bit tensor peak,
   // prepared 0.23 against 0.29): the step time is set by the fold warps' accumulator round trip, which the
   // pair leaves unchanged, and every hand-over now crosses two SMs.  Kept selectable for A/B runs.
-  const bool pair = pair_selected() && pp::supported(a.T, a.K, a.N) && (!f8 || prep);
+  const bool pair = pair_selected() && !(a.flags & W4A4_FLAG_TILES_128) && pp::supported(a.T, a.K, a.N) && (!f8 || prep);
   cudaError_t e;
   if (wide_kernel) {
     p.band = (p.band + 1) / 2;                  // tiles twice as wide
@@ -671,6 +696,8 @@ int run_gemm(GemmArgs& a) {
   if ((long long)a.T > 16LL * 65535) return fail(W4A4_ERR_UNSUPPORTED, "T=%d exceeds the grid limit", a.T);
   DeviceInfo* dev = nullptr;
   rc = current_device(&dev);
+  if (rc) return rc;
+  rc = check_tile_flags(a.flags);
   if (rc) return rc;
   if ((a.flags & W4A4_FLAG_FORCE_TENSOR) && !w4a4::pre::supported(a.T, a.K, a.N))
     return fail(W4A4_ERR_UNSUPPORTED, "tensor-core path does not support T=%d K=%d N=%d", a.T, a.K, a.N);
@@ -956,11 +983,13 @@ int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared, int*
   int rc = check_common(T, K, N, nnz);
   if (rc) return rc;
   CHECK_ARG(kernel && code_format, "NULL output pointer");
+  rc = check_tile_flags(flags);
+  if (rc) return rc;
   DeviceInfo* dev = nullptr;
   rc = current_device(&dev);
   if (rc) return rc;
   const GemmChoice c = wants_tensor_path(T, K, N, flags, dev->sm_count, prepared != 0)
-                           ? choose_tensor_kernel(T, K, N, prepared != 0, true, dev->sm_count)
+                           ? choose_tensor_kernel({T, K, N, true, nnz}, flags, prepared != 0, true, dev->sm_count)
                            : GemmChoice{W4A4_KERNEL_STREAM, W4A4_CODES_S8};
   *kernel = c.kernel;
   *code_format = c.codes;
@@ -1176,10 +1205,12 @@ int w4a4_fused_quant_dense_sparse_prepared(const void* X, long long ldx, const i
   a.nnz = nnz; a.do_dense = true; a.sparse_weight = 16.f;
   // the quantiser writes the codes in the format the GEMM kernel of this call will read
   a.W_low_prep = W_low_prepared; a.W_high_prep = W_high_prepared;
+  rc = check_tile_flags(flags);
+  if (rc) return rc;
   const bool tensor = wants_tensor_path(T, K, N, flags, dev->sm_count, has_prepared(a));
   if (!tensor || !has_prepared(a)) a.W_low_prep = a.W_high_prep = nullptr;
   // what the chosen tensor-core kernel reads; the streaming kernel reads s8 codes
-  a.xe_fmt = tensor ? choose_tensor_kernel(T, K, N, has_prepared(a), true, dev->sm_count).codes : W4A4_CODES_S8;
+  a.xe_fmt = tensor ? choose_tensor_kernel({T, K, N, true, nnz}, flags, has_prepared(a), true, dev->sm_count).codes : W4A4_CODES_S8;
   a.widen = tensor && !has_prepared(a) && a.xe_fmt == W4A4_CODES_E4M3;
   rc = launch_quant(X, ldx, perm, nullptr, ws + wl.scale_x, nullptr, ws + wl.xe, reinterpret_cast<float*>(ws + wl.sumxf),
                     T, K, s, dev->sm_count, a.xe_fmt);

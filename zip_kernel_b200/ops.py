@@ -217,8 +217,12 @@ def _flags(token_major: bool, force: Optional[str]) -> int:
         f |= _lib.FLAG_FORCE_STREAM
     elif force == "tensor":
         f |= _lib.FLAG_FORCE_TENSOR
+    elif force == "tensor128":
+        f |= _lib.FLAG_FORCE_TENSOR | _lib.FLAG_TILES_128
+    elif force == "tensor256":
+        f |= _lib.FLAG_FORCE_TENSOR | _lib.FLAG_TILES_256
     elif force is not None:
-        raise ValueError(f"force must be None, 'stream' or 'tensor', got {force!r}")
+        raise ValueError(f"force must be None, 'stream', 'tensor', 'tensor128' or 'tensor256', got {force!r}")
     return f
 
 
