@@ -143,3 +143,32 @@ def test_tile_choice(T, N, K, nnz, prepared, wide):
         pytest.skip("the expected choices are those of 148 SMs")
     want = _lib.KERNEL_TILES_256 if wide else _lib.KERNEL_TILES_128
     assert ops.gemm_choice(T, N, K, nnz, prepared=prepared, force="tensor")[0] == want
+
+
+# outputs whose rows start at every remainder of 16 bytes, in both layouts and with an unaligned base; nothing around them is touched
+@pytest.mark.parametrize("T,N", [(256 + r, 128 + r) for r in range(1, 9)] + [(1, 131), (2, 1), (129, 257), (8, 3), (1000, 260), (520, 129)])
+@pytest.mark.parametrize("base_off", [0, 1, 4])
+def test_stores_of_unaligned_rows(T, N, base_off):
+    from zip_kernel_b200 import _lib, ops
+    lib, dev = _lib.load(), torch.device("cuda")
+    K = 256
+    W, X = make_case(T, N, K, 0.3)
+    Wd = W.to(dev)
+    q = ops.activation_quant_cuda(X.to(dev), Wd.perm)
+    ws = _lib.workspace(dev, T, K, N, Wd.n_hp_blocks)
+    nnz = Wd.n_hp_blocks
+
+    def call(flags):
+        buf = torch.full((T * N + 32,), 7.0, dtype=torch.float16, device=dev)
+        Y = buf[8 + base_off:8 + base_off + T * N]
+        rc = lib.w4a4_fused_dense_sparse(
+            Wd.W_low_packed.data_ptr(), Wd.W_high_blocks_packed.data_ptr() if nnz else None, Wd.hp_row_offsets.data_ptr(),
+            Wd.hp_col_indices.data_ptr() if nnz else None, q[0].data_ptr(), Wd.scale_u4.data_ptr(), Wd.zero_u4.data_ptr(), q[2].data_ptr(),
+            q[1].data_ptr(), Y.data_ptr(), T, K, N, nnz, flags | _lib.FLAG_FORCE_TENSOR, ws.data_ptr(), ws.numel(),
+            torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, lib.w4a4_last_error()
+        assert bool((buf[:8 + base_off] == 7.0).all()) and bool((buf[8 + base_off + T * N:] == 7.0).all())
+        return Y
+    for layout in (0, _lib.FLAG_OUT_TOKEN_MAJOR):
+        assert torch.equal(call(layout | _lib.FLAG_TILES_256), call(layout | _lib.FLAG_TILES_128))
+    assert _lib.device_error(dev) == 0

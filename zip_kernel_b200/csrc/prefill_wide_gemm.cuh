@@ -121,6 +121,20 @@ __device__ __forceinline__ bool wait_suspend(uint64_t* bar, uint32_t parity, int
   return false;
 }
 
+// `count` <= 32 * P neighbouring outputs that may start at any element, by one warp.  Straight-line code, all reads before
+// the first store: 4-byte stores between single elements need half as many, and branches that take longer.
+// Measured, 2048 tokens 4096 -> 28673 prepared, token-major: 8 single halves per thread, 16 bytes apart, 460 us; a
+// loop of 2-byte stores 390; 4-byte stores with branches 402; this 341 (28672: 335).
+template <int P>
+__device__ __forceinline__ void store_run(__half* dst, uint32_t src, int count, int lane, const float (&scale)[P]) {
+  float v[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) v[k] = lds_f1(src + (lane + 32 * k) * 4);
+#pragma unroll
+  for (int k = 0; k < P; ++k)
+    if (lane + 32 * k < count) dst[lane + 32 * k] = __float2half_rn(v[k] * scale[k]);
+}
+
 template <bool PREP>
 __global__ void __launch_bounds__(THREADS, 1)
 prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_wh,
@@ -481,6 +495,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     // The ring has no copy or MMA in flight any more: it takes the tile's sums, in the order the output has in
     // memory, and a rolled loop of 16-byte stores drains them (storing straight from the registers is 128
     // two-byte stores per thread and several times the code, executed once: about 12000 clk on this tile).
+    // Where the output's rows do not all start on 16 bytes, a warp stores a row of the tile at a time (store_run).
     const uint32_t stage = smem_u32(sm);
     asm volatile("bar.sync 1, %0;" ::"n"(N_FOLD * 32) : "memory");       // every fold warp has seen the last MMAs complete
     if (p.y_stride_n == 1) {
@@ -489,18 +504,23 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       for (int i = 0; i < COLS; ++i) sts_f1(stage + ((c0 + i) * ROWS + rl) * 4, y[i]);
       asm volatile("bar.sync 1, %0;" ::"n"(N_FOLD * 32) : "memory");
       const bool vec = (p.y_stride_t & 7) == 0 && (reinterpret_cast<uintptr_t>(p.Y) & 15) == 0;
+      if (!vec) {
+        const int count = min(ROWS, p.N - row0);
+#pragma unroll 2
+        for (int t = warp - WARP_FOLD0; ok && t < live; t += N_FOLD) {
+          const float sx[ROWS / 32] = {sxs[t], sxs[t], sxs[t], sxs[t]};
+          store_run<ROWS / 32>(p.Y + (size_t)(tok0 + t) * p.y_stride_t + row0, stage + t * ROWS * 4, count, lane, sx);
+        }
+      }
 #pragma unroll 1
-      for (int i = ft; ok && i < live * (ROWS / 8); i += N_FOLD * 32) {
+      for (int i = ft; vec && ok && i < live * (ROWS / 8); i += N_FOLD * 32) {
         const int t = i >> 4, r8 = (i & 15) * 8;
         const float4 u = lds_f4(stage + (t * ROWS + r8) * 4), v = lds_f4(stage + (t * ROWS + r8 + 4) * 4);
         const float sx = sxs[t];
         __align__(16) __half2 h[4] = {__floats2half2_rn(u.x * sx, u.y * sx), __floats2half2_rn(u.z * sx, u.w * sx),
                                       __floats2half2_rn(v.x * sx, v.y * sx), __floats2half2_rn(v.z * sx, v.w * sx)};
-        __half* dst = p.Y + (size_t)(tok0 + t) * p.y_stride_t + row0 + r8;
-        if (vec && row0 + r8 + 8 <= p.N) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(h);
-        else
-          for (int e = 0; e < 8; ++e)
-            if (row0 + r8 + e < p.N) dst[e] = reinterpret_cast<__half*>(h)[e];
+        // (the stride, N, is a multiple of 8: no ragged eight)
+        if (row0 + r8 < p.N) *reinterpret_cast<uint4*>(p.Y + (size_t)(tok0 + t) * p.y_stride_t + row0 + r8) = *reinterpret_cast<uint4*>(h);
       }
     } else {
       // row-major: [row][TN tokens], consecutive rows 4 banks apart
@@ -511,19 +531,24 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
       asm volatile("bar.sync 1, %0;" ::"n"(N_FOLD * 32) : "memory");
       const bool vec = (p.y_stride_n & 7) == 0 && (reinterpret_cast<uintptr_t>(p.Y) & 15) == 0;
       const int rows = min(ROWS, p.N - row0);
+      if (!vec) {
+        float sx[TN / 32];
+#pragma unroll
+        for (int k = 0; k < TN / 32; ++k) sx[k] = sxs[lane + 32 * k];
+#pragma unroll 2
+        for (int q = warp - WARP_FOLD0; ok && q < rows; q += N_FOLD)
+          store_run<TN / 32>(p.Y + (size_t)(row0 + q) * p.y_stride_n + tok0, stage + q * PITCH * 4, live, lane, sx);
+      }
 #pragma unroll 1
-      for (int i = ft; ok && i < rows * (TN / 8); i += N_FOLD * 32) {
+      for (int i = ft; vec && ok && i < rows * (TN / 8); i += N_FOLD * 32) {
         const int q = i / (TN / 8), t8 = (i % (TN / 8)) * 8;
         if (t8 >= live) continue;
         const float4 u = lds_f4(stage + (q * PITCH + t8) * 4), v = lds_f4(stage + (q * PITCH + t8 + 4) * 4);
         const float4 a = lds_f4(smem_u32(sxs + t8)), b = lds_f4(smem_u32(sxs + t8 + 4));
         __align__(16) __half2 h[4] = {__floats2half2_rn(u.x * a.x, u.y * a.y), __floats2half2_rn(u.z * a.z, u.w * a.w),
                                       __floats2half2_rn(v.x * b.x, v.y * b.y), __floats2half2_rn(v.z * b.z, v.w * b.w)};
-        __half* dst = p.Y + (size_t)(row0 + q) * p.y_stride_n + tok0 + t8;
-        if (vec && t8 + 8 <= live) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(h);
-        else
-          for (int e = 0; e < 8; ++e)
-            if (t8 + e < live) dst[e] = reinterpret_cast<__half*>(h)[e];
+        // (the stride, T, is a multiple of 8: no ragged eight)
+        *reinterpret_cast<uint4*>(p.Y + (size_t)(row0 + q) * p.y_stride_n + tok0 + t8) = *reinterpret_cast<uint4*>(h);
       }
     }
   }
