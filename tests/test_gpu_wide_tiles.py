@@ -132,17 +132,20 @@ def test_tile_flags_are_checked():
         ops.gemm_choice(T, N, K, force="wide")
 
 
-# (tokens, d_out, d_in, residual blocks, prepared, 256-token tiles): the measured winner on 148 SMs
-@pytest.mark.parametrize("T,N,K,nnz,prepared,wide", [
-    (384, 6144, 256, 5, False, False), (512, 4096, 512, 6, False, False), (384, 6144, 128, 2, True, False), (128, 4096, 512, 6, False, True),
-    (192, 4096, 256, 3, True, True), (512, 28672, 14336, 1254, True, False), (512, 4096, 14336, 179, True, False), (600, 4096, 14336, 179, True, True),
-    (1024, 6144, 4096, 77, False, False), (1024, 6144, 4096, 77, True, True), (2048, 28672, 4096, 358, False, True)])
-def test_tile_choice(T, N, K, nnz, prepared, wide):
+# (tokens, d_out, d_in, residual blocks, prepared, token-major, 256-token tiles): the measured winner on 148 SMs
+@pytest.mark.parametrize("T,N,K,nnz,prepared,token_major,wide", [
+    (384, 6144, 256, 5, False, True, False), (512, 4096, 512, 6, False, True, False), (384, 6144, 128, 2, True, True, False),
+    (128, 4096, 512, 6, False, True, True), (192, 4096, 256, 3, True, True, True), (512, 28672, 14336, 1254, True, True, False),
+    (512, 4096, 14336, 179, True, True, False), (600, 4096, 14336, 179, True, True, True), (1024, 6144, 4096, 77, False, True, False),
+    (1024, 6144, 4096, 77, True, True, True), (2048, 28672, 4096, 358, False, True, True),
+    (256, 4096, 4096, 51, True, False, False), (257, 4096, 4096, 51, True, False, True), (257, 4096, 4096, 51, True, True, False),
+    (257, 4096, 14336, 179, False, False, False), (104, 336, 640, 1, True, False, True), (128, 336, 640, 1, True, False, False)])
+def test_tile_choice(T, N, K, nnz, prepared, token_major, wide):
     from zip_kernel_b200 import _lib, ops
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the expected choices are those of 148 SMs")
     want = _lib.KERNEL_TILES_256 if wide else _lib.KERNEL_TILES_128
-    assert ops.gemm_choice(T, N, K, nnz, prepared=prepared, force="tensor")[0] == want
+    assert ops.gemm_choice(T, N, K, nnz, prepared=prepared, token_major=token_major, force="tensor")[0] == want
 
 
 # outputs whose rows start at every remainder of 16 bytes, in both layouts and with an unaligned base; nothing around them is touched

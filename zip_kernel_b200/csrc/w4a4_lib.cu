@@ -412,30 +412,42 @@ bool pair_selected() {
   return e && atoi(e) != 0;
 }
 
-// Sizes that a choice of kernel goes by: `dense` groups of K in every block-row, `nnz` residual blocks over all.
+// What a choice of kernel goes by: `dense` groups of K in every block-row, `nnz` residual blocks over all, and the
+// layout of the output.
 struct GemmSizes {
   int T, K, N;
   bool dense;
   int nnz;
+  bool token_major;
 };
 
 // Tiles of 256 tokens (prefill_wide_gemm_kernel) or of 128 (prefill_gemm_kernel)?  Both run one CTA per SM, so a launch
-// takes waves x (K-steps x step + fixed), the steps counted with the residual blocks.  The constants (us) were
-// fitted on B200 at 1.9 GHz to the measured winner of 254 launches whose waves differ (d_in 128 to 14336, d_out
-// 1024 to 28672, 64 to 2048 tokens, 0 / 5 / 15 % residual blocks, residual-only calls): none of them loses more
-// than 1 %.  Near the line: 14336 -> 4096, 600 tokens, prepared (1 against 2 waves) 109 against 113 us; 14336 -> 28672,
-// 512 tokens, prepared (4 against 7) 380 against 355 us; 4096 -> 6144, 1024 tokens, packed (2 against 3) 83 against 81.
-// With equally many waves the narrow tile's shorter steps win (14336 -> 4096, 512 tokens, prepared 105 against 64 us; 256 ->
-// 6144, 384 tokens, packed 12.6 against 10.7; 15 % blocks of 4096 -> 4096 alone, 512 tokens 18.2 against 15.5), except
-// where a few steps of few tokens leave mostly the fixed part (512 -> 4096, 128 tokens, packed 10.7 against 11.4
-// us; 256 -> 4096, 192 tokens, prepared 8.5 against 9.0).
+// takes waves x (K-steps x step + fixed), the steps counted with the residual blocks.  The constants (us) are fitted to
+// the winner of about 2000 launches with each kernel forced on B200 at 1.9 GHz (d_in 128 to 16384, d_out 300 to
+// 40000, 64 to 4096 tokens, 0 / 5 / 15 % residual blocks, residual-only calls, odd and even sizes, both layouts); of 771
+// launches whose waves differ 5 are more than 3 % behind the better kernel, one more than 7 %.  Near the line:
+// 14336 -> 4096, 600 tokens, prepared (1 wave against 2) 109 against 113 us; 14336 -> 28672, 512 tokens, prepared (4
+// against 7) 380 against 355; 4096 -> 6144, 1024 tokens, packed (2 against 3) 83 against 81.
+// With equally many waves the narrow tile's shorter steps win (14336 -> 4096, 512 tokens, prepared 105 against 64 us),
+// except where mostly the fixed part is left, a few steps of few tokens (512 -> 4096, 128 tokens, packed 10.7 against
+// 11.4; 256 -> 4096, 192 tokens, prepared 8.5 against 9.0).
+// Row-major outputs the narrow kernel stores 64 tokens of a row at a time, with 16-byte stores where these 64 exist and
+// start on 16 bytes and with 2-byte stores scattered over 32 rows where not: every wave of T % 8 != 0 (4096 ->
+// 4096, 2047 tokens, prepared 64 against 141), the last token tile of T % 64 != 0 (640 -> 336, 104 tokens, prepared 10
+// against 14).  The wide kernel stages its stores, so it wins there up to more steps.
 bool wants_wide_tiles(const GemmSizes& z, bool prepared, int sm_count) {
   const long long rows = (z.N + 127) / 128;
   const long long w256 = (rows * ((z.T + 255) / 256) + sm_count - 1) / sm_count;
   const long long w128 = (rows * ((z.T + 127) / 128) + sm_count - 1) / sm_count;
-  if (w256 == w128) return z.dense && ((z.T <= 128 && z.K <= 512) || (prepared && z.T <= 256 && z.K <= 256));
   const double n = (z.dense ? z.K / 128 : 0) + (double)z.nnz / (double)rows;
-  return prepared ? w256 * (0.72 * n + 3.0) <= w128 * (0.37 * n + 6.5) : w256 * (0.94 * n + 3.5) <= w128 * (0.55 * n + 4.5);
+  const bool scattered = !z.token_major && z.T % 8 != 0, scattered_end = !z.token_major && z.T % 64 != 0;
+  if (w256 == w128) {
+    if (scattered) return n <= (prepared ? 60 : 34);
+    if (scattered_end) return n <= (prepared ? 16 : 2.5);
+    return z.token_major && z.dense && ((z.T <= 128 && z.K <= 512) || (prepared && z.T <= 256 && z.K <= 384));
+  }
+  return prepared ? w256 * (0.74 * n + 2.5) <= w128 * (0.37 * n + (scattered ? 18.0 : 7.0))
+                  : w256 * (1.04 * n + 2.5) <= w128 * (0.55 * n + (scattered ? 16.0 : 4.5));
 }
 
 struct GemmChoice {
@@ -484,7 +496,7 @@ int launch_prefill(const GemmArgs& a_in, DeviceInfo* dev) {
   // widened to s8 (integer MMAs).  When the library expands the codes itself choose_tensor_kernel picks.
   const bool dump = a.acc_dump || a.acc_hi_dump;
   const bool has_sparse = a.nnz > 0 && a.sparse_weight != 0.f;
-  const GemmSizes sizes{a.T, a.K, a.N, a.do_dense, has_sparse ? a.nnz : 0};
+  const GemmSizes sizes{a.T, a.K, a.N, a.do_dense, has_sparse ? a.nnz : 0, (a.flags & W4A4_FLAG_OUT_TOKEN_MAJOR) != 0};
   if (a.XE == nullptr) {
     a.xe_fmt = prep   ? W4A4_CODES_E4M3
                : dump ? ((a.flags & W4A4_FLAG_CODES_E4M3_PACKED) ? W4A4_CODES_E4M3_PACKED : W4A4_CODES_S8)
@@ -989,7 +1001,8 @@ int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared, int*
   rc = current_device(&dev);
   if (rc) return rc;
   const GemmChoice c = wants_tensor_path(T, K, N, flags, dev->sm_count, prepared != 0)
-                           ? choose_tensor_kernel({T, K, N, true, nnz}, flags, prepared != 0, true, dev->sm_count)
+                           ? choose_tensor_kernel({T, K, N, true, nnz, (flags & W4A4_FLAG_OUT_TOKEN_MAJOR) != 0}, flags, prepared != 0,
+                                                  true, dev->sm_count)
                            : GemmChoice{W4A4_KERNEL_STREAM, W4A4_CODES_S8};
   *kernel = c.kernel;
   *code_format = c.codes;
@@ -1210,7 +1223,9 @@ int w4a4_fused_quant_dense_sparse_prepared(const void* X, long long ldx, const i
   const bool tensor = wants_tensor_path(T, K, N, flags, dev->sm_count, has_prepared(a));
   if (!tensor || !has_prepared(a)) a.W_low_prep = a.W_high_prep = nullptr;
   // what the chosen tensor-core kernel reads; the streaming kernel reads s8 codes
-  a.xe_fmt = tensor ? choose_tensor_kernel({T, K, N, true, nnz}, flags, has_prepared(a), true, dev->sm_count).codes : W4A4_CODES_S8;
+  a.xe_fmt = tensor ? choose_tensor_kernel({T, K, N, true, nnz, (flags & W4A4_FLAG_OUT_TOKEN_MAJOR) != 0}, flags, has_prepared(a),
+                                           true, dev->sm_count).codes
+                    : W4A4_CODES_S8;
   a.widen = tensor && !has_prepared(a) && a.xe_fmt == W4A4_CODES_E4M3;
   rc = launch_quant(X, ldx, perm, nullptr, ws + wl.scale_x, nullptr, ws + wl.xe, reinterpret_cast<float*>(ws + wl.sumxf),
                     T, K, s, dev->sm_count, a.xe_fmt);

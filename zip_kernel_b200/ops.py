@@ -119,11 +119,11 @@ def _code_flag(e4m3) -> int:
 
 
 def gemm_choice(T: int, d_out: int, d_in: int, n_hp_blocks: int = 0, *, prepared: bool = False,
-                force: Optional[str] = None, device=None) -> Tuple[int, int]:
+                force: Optional[str] = None, token_major: bool = False, device=None) -> Tuple[int, int]:
     """``(kernel, code format)`` (``_lib.KERNEL_*``, ``_lib.CODES_*``) of a fused call with these sizes on ``device``."""
     kernel, codes = ctypes.c_int(0), ctypes.c_int(0)
     with _lib.on_device(torch.device("cuda") if device is None else device):
-        _lib.check(_L.w4a4_gemm_choice(int(T), int(d_in), int(d_out), int(n_hp_blocks), _flags(False, force), int(prepared),
+        _lib.check(_L.w4a4_gemm_choice(int(T), int(d_in), int(d_out), int(n_hp_blocks), _flags(token_major, force), int(prepared),
                                        ctypes.byref(kernel), ctypes.byref(codes)), "gemm_choice")
     return kernel.value, codes.value
 

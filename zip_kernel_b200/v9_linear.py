@@ -85,7 +85,7 @@ def _wants_e4m3(W: V9WeightContainer, T: int):
     # and narrow tiles give the same bits.
     if T < 64:                                       # always streamed against s8 codes
         return False
-    codes = ops.gemm_choice(T, W.d_out, W.d_in, W.n_hp_blocks, prepared=W.prepared is not None,
+    codes = ops.gemm_choice(T, W.d_out, W.d_in, W.n_hp_blocks, prepared=W.prepared is not None, token_major=True,
                             device=W.W_low_packed.device)[1]
     if codes == _lib.CODES_E4M3_PACKED:
         return "packed"
