@@ -111,15 +111,14 @@ size_t w4a4_workspace_bytes(int T, int K, int N, int nnz);
 
 /* The kernel that w4a4_fused_quant_dense_sparse (prepared = 0) or its _prepared form (prepared = 1: for every
  * operand in use) runs on the current device for these sizes and flags, and the W4A4_CODES_* form it expands
- * the activations to.  Host only, no counterpart in the reference.  A caller that expands activations itself
+ * the activations to: W4A4_KERNEL_* | form << 8, or minus an error code.  Host only, no counterpart in the reference.  A caller that expands activations itself
  * gets the same output bits from W4A4_CODES_S8 wherever this reports W4A4_CODES_E4M3 without prepared weights:
  * the *_expanded entry points read natural-order e4m3 codes against prepared weights only. */
 #define W4A4_KERNEL_STREAM    0   /* weight-streaming split-K kernel */
 #define W4A4_KERNEL_TILES_128 1   /* tensor-core kernel, 128-token tiles */
 #define W4A4_KERNEL_TILES_256 2   /* tensor-core kernel, 256-token tiles */
 #define W4A4_KERNEL_PAIRS     3   /* tensor-core kernel on CTA pairs (W4A4_PREFILL_PAIR=1) */
-int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared, int* kernel /* host */,
-                     int* code_format /* host */);
+int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared);
 
 /* Replaces fused_dense_sparse_mma_int4_launch, fused_gemv_decode_launch and
  * fused_gemv_smallT_launch (bindings.cc:187-235; kernels

@@ -41,7 +41,7 @@ SIGNATURES = {
     "w4a4_peer_close": (_INT, [_PTR]),
     "w4a4_peer_push_wait": (_INT, [_PTR, _LL, _c.POINTER(_PTR), _c.POINTER(_PTR), _LL, _LL, _INT, _INT, _INT, _INT, _PTR, _INT, _PTR]),
     "w4a4_workspace_bytes": (_SZ, [_INT, _INT, _INT, _INT]),
-    "w4a4_gemm_choice": (_INT, [_INT] * 6 + [_c.POINTER(_INT)] * 2),
+    "w4a4_gemm_choice": (_INT, [_INT] * 6),
     "w4a4_fused_dense_sparse": (_INT, [_PTR] * 10 + [_INT] * 5 + [_PTR, _SZ, _PTR]),
     "w4a4_expanded_codes_bytes": (_SZ, [_INT, _INT]),
     "w4a4_expanded_sums_bytes": (_SZ, [_INT, _INT]),

@@ -990,23 +990,17 @@ size_t w4a4_workspace_bytes(int T, int K, int N, int nnz) {
   return ws_layout(T, K).total;
 }
 
-int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared, int* kernel, int* code_format) {
+int w4a4_gemm_choice(int T, int K, int N, int nnz, int flags, int prepared) {
   begin_call();
   int rc = check_common(T, K, N, nnz);
-  if (rc) return rc;
-  CHECK_ARG(kernel && code_format, "NULL output pointer");
-  rc = check_tile_flags(flags);
-  if (rc) return rc;
+  if (rc == 0) rc = check_tile_flags(flags);
   DeviceInfo* dev = nullptr;
-  rc = current_device(&dev);
-  if (rc) return rc;
-  const GemmChoice c = wants_tensor_path(T, K, N, flags, dev->sm_count, prepared != 0)
-                           ? choose_tensor_kernel({T, K, N, true, nnz, (flags & W4A4_FLAG_OUT_TOKEN_MAJOR) != 0}, flags, prepared != 0,
-                                                  true, dev->sm_count)
-                           : GemmChoice{W4A4_KERNEL_STREAM, W4A4_CODES_S8};
-  *kernel = c.kernel;
-  *code_format = c.codes;
-  return W4A4_OK;
+  if (rc == 0) rc = current_device(&dev);
+  if (rc) return -rc;
+  if (!wants_tensor_path(T, K, N, flags, dev->sm_count, prepared != 0)) return W4A4_KERNEL_STREAM | W4A4_CODES_S8 << 8;
+  const GemmChoice c = choose_tensor_kernel({T, K, N, true, nnz, (flags & W4A4_FLAG_OUT_TOKEN_MAJOR) != 0}, flags, prepared != 0, true,
+                                            dev->sm_count);
+  return c.kernel | c.codes << 8;
 }
 
 int w4a4_fused_dense_sparse(const void* W_low, const void* W_high, const int32_t* hp_row_offsets,

@@ -13,7 +13,6 @@ Differences that follow from the B200 design (results are unaffected):
 
 from __future__ import annotations
 
-import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -121,11 +120,11 @@ def _code_flag(e4m3) -> int:
 def gemm_choice(T: int, d_out: int, d_in: int, n_hp_blocks: int = 0, *, prepared: bool = False,
                 force: Optional[str] = None, token_major: bool = False, device=None) -> Tuple[int, int]:
     """``(kernel, code format)`` (``_lib.KERNEL_*``, ``_lib.CODES_*``) of a fused call with these sizes on ``device``."""
-    kernel, codes = ctypes.c_int(0), ctypes.c_int(0)
     with _lib.on_device(torch.device("cuda") if device is None else device):
-        _lib.check(_L.w4a4_gemm_choice(int(T), int(d_in), int(d_out), int(n_hp_blocks), _flags(token_major, force), int(prepared),
-                                       ctypes.byref(kernel), ctypes.byref(codes)), "gemm_choice")
-    return kernel.value, codes.value
+        choice = _L.w4a4_gemm_choice(int(T), int(d_in), int(d_out), int(n_hp_blocks), _flags(token_major, force), int(prepared))
+    if choice < 0:
+        _lib.check(-choice, "gemm_choice")
+    return choice & 0xff, choice >> 8
 
 
 def _fused_prologue(which: str, X2: torch.Tensor, K: int, perm, norm_weight, eps: float, expanded: bool, e4m3):
@@ -147,7 +146,7 @@ def _fused_prologue(which: str, X2: torch.Tensor, K: int, perm, norm_weight, eps
     pp = None if perm is None else perm.data_ptr()
     with _lib.on_device(dev):
         if which == "rmsnorm":
-            w = norm_weight.to(device=dev, dtype=torch.float16).contiguous()
+            w = _cd(norm_weight if norm_weight.device == dev else norm_weight.to(dev), torch.float16)
             _lib.check(_L.w4a4_rmsnorm_quant(X2.data_ptr(), X2.stride(0) if T > 1 else K, w.data_ptr(), float(eps), pp, *outs,
                                              _code_format(e4m3), T, K, _lib.stream_ptr(dev)), "rmsnorm_quant")
         else:
@@ -448,13 +447,12 @@ def fused_dense_sparse_expanded_cuda(
     sx = _cd(scale_x, torch.float16)
     Y = _out(d_out, T, W.device, token_major)
     with _lib.on_device(W.device):
-        ws = _lib.workspace(W.device, T, d_in, d_out, nnz)
         plo, phi = _prepared_ptrs(prepared, W, Wh, nnz)
         _lib.check(_L.w4a4_fused_dense_sparse_expanded_prepared(
             W.data_ptr(), Wh.data_ptr() if nnz else None, plo, phi, ro.data_ptr(), ci.data_ptr() if nnz else None,
             XE.data_ptr(), sumxf.data_ptr(), s.data_ptr(), z.data_ptr(), sx.data_ptr(), Y.data_ptr(),
             T, d_in, d_out, nnz, _flags(token_major, force) | _code_flag(e4m3),
-            ws.data_ptr(), ws.numel(), _lib.stream_ptr(W.device)), "fused_dense_sparse_expanded")
+            None, 0, _lib.stream_ptr(W.device)), "fused_dense_sparse_expanded")     # (XE is all the scratch there is)
     return Y
 
 

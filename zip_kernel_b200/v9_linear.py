@@ -22,6 +22,8 @@ from .pack_utils import BCOL, V9WeightContainer, unpack_s4_le
 
 DECODE_T_THRESHOLD = 128
 
+_L = _lib.load()
+
 
 # W4A16 route for long prompts (the reference's backend/dispatcher.py:228-238): a layer WITHOUT residual blocks at
 # T >= 1024 (or T >= 512 on shapes up to 4096 x 4096) is dequantised to fp16 and multiplied by a library fp16 GEMM;
@@ -80,16 +82,21 @@ def _gemm_on_expanded(quantised, W: V9WeightContainer, lead_shape, e4m3) -> torc
 
 
 def _wants_e4m3(W: V9WeightContainer, T: int):
-    # The codes v9_linear_forward would use for this many tokens, so that both round alike.  Where it runs wide tiles
-    # on packed weights (natural-order e4m3 codes that only a prepared copy can be read against here), s8 codes
-    # and narrow tiles give the same bits.
-    if T < 64:                                       # always streamed against s8 codes
+    # The codes v9_linear_forward would use for this many tokens, so that both round alike: below 64 tokens it streams,
+    # from 256 on it never does, else (and for W4A4_PREFILL_F8) the library knows.  Where it runs wide tiles on
+    # packed weights (natural-order e4m3 codes that only a prepared copy can be read against here), s8 codes and
+    # narrow tiles give the same bits.
+    if T < 64:
         return False
-    codes = ops.gemm_choice(T, W.d_out, W.d_in, W.n_hp_blocks, prepared=W.prepared is not None, token_major=True,
-                            device=W.W_low_packed.device)[1]
-    if codes == _lib.CODES_E4M3_PACKED:
-        return "packed"
-    return codes == _lib.CODES_E4M3 and W.prepared is not None
+    prepared = W.prepared is not None
+    if prepared and T >= 256:
+        return True
+    # (blocks and device only matter to the tile, not to the codes: left out, the call is on the host path of small layers)
+    choice = _L.w4a4_gemm_choice(T, W.d_in, W.d_out, 0, _lib.FLAG_OUT_TOKEN_MAJOR, prepared)
+    if choice < 0:
+        _lib.check(-choice, "gemm_choice")
+    codes = choice >> 8
+    return "packed" if codes == _lib.CODES_E4M3_PACKED else prepared and codes == _lib.CODES_E4M3
 
 
 def v9_linear_forward_rmsnorm(X_fp16: torch.Tensor, norm_weight: torch.Tensor, eps: float,
