@@ -614,6 +614,25 @@ def leg_stack(device):
 
 
 # ----------------------------------------------------------------------------- main
+def headline(out):
+    """The line that is printed on stdout: the record without its legs and long texts, floats to six digits, so that
+    it stays well under 2 kB."""
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.6g}")
+        return {k: short(x) for k, x in v.items()} if isinstance(v, dict) else v
+
+    parts = {"config": ("workload", "l2", "parallelism", "weights"), "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step"),
+             "roofline": ("bound", "achieved", "peak", "unit", "frac", "kernel"), "cpu_baseline": ("value", "unit", "cores", "kind")}
+    line = {}
+    for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline", "dtype",
+              "data", "config", "e2e", "gpu_launches", "roofline", "clocks", "cpu_baseline", "decode_tok_s", "sharded_parity", "device_error_word",
+              "device_error_word_after_legs", "wall_s"):
+        if k in out:
+            line[k] = short({p: out[k][p] for p in parts[k] if p in out[k]} if k in parts else out[k])
+    return line
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -810,7 +829,9 @@ def main():
                                "sample": f"one pass over all {len(items)} linears of the workload ({dt:.1f} s) after one warm-up linear; {how}"}
     out["wall_s"] = time.perf_counter() - t_start
     if rank == 0:
-        print(json.dumps(out), flush=True)
+        # the whole record first, on the other stream: a reader of the last few kB of stdout gets the headline complete
+        print(json.dumps(out), file=sys.stderr, flush=True)
+        print(json.dumps(headline(out)), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
