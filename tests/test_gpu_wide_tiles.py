@@ -131,12 +131,13 @@ def test_tile_flags_are_checked():
 
 # (tokens, d_out, d_in, residual blocks, prepared, token-major, 256-token tiles): the measured winner on 148 SMs
 @pytest.mark.parametrize("T,N,K,nnz,prepared,token_major,wide", [
-    (384, 6144, 256, 5, False, True, False), (512, 4096, 512, 6, False, True, False), (384, 6144, 128, 2, True, True, False),
-    (128, 4096, 512, 6, False, True, True), (192, 4096, 256, 3, True, True, True), (512, 28672, 14336, 1254, True, True, False),
+    (384, 6144, 256, 5, False, True, False), (512, 4096, 512, 6, False, True, False), (512, 4096, 1024, 13, True, True, False),
+    (128, 4096, 512, 6, False, True, True), (192, 4096, 256, 3, True, True, True), (384, 28672, 4096, 358, True, True, False),
     (512, 4096, 14336, 179, True, True, False), (600, 4096, 14336, 179, True, True, True), (1024, 6144, 4096, 77, False, True, False),
     (1024, 6144, 4096, 77, True, True, True), (2048, 28672, 4096, 358, False, True, True),
     (256, 4096, 4096, 51, True, False, False), (257, 4096, 4096, 51, True, False, True), (257, 4096, 4096, 51, True, True, False),
-    (257, 4096, 14336, 179, False, False, False), (104, 336, 640, 1, True, False, True), (128, 336, 640, 1, True, False, False)])
+    (257, 4096, 14336, 179, False, False, False), (104, 336, 640, 1, True, False, True), (128, 336, 640, 1, True, False, False),
+    (112, 592, 384, 2, False, False, True), (776, 1024, 512, 2, False, False, False)])
 def test_tile_choice(T, N, K, nnz, prepared, token_major, wide):
     from zip_kernel_b200 import _lib, ops
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:

@@ -77,20 +77,6 @@ __device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
 // instruction descriptors without the token count (bits 17..22: N / 8), M = 128
 constexpr uint32_t IDESC_F8_M = (1u << 4) | ((uint32_t)(ROWS >> 4) << 24);
 constexpr uint32_t IDESC_TF32_M = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(ROWS >> 4) << 24);
-__device__ __forceinline__ void umma_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 
 // Bounded wait whose polls may sleep in hardware (up to 20 us each): the roles of this kernel wait for hundreds of
 // clocks at a time, and polling takes issue slots and instruction fetches from the fold warps of the same
@@ -257,7 +243,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         const uint64_t off = (uint64_t)(s * (SLOT >> 4));
         const uint32_t d = tmem_base + buf * TN;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma_f8(d, a0 + off + 2 * j, b0 + off + 2 * j, IDESC_F8_M | ncol, j > 0);
+        for (int j = 0; j < 4; ++j) pre::umma_f8(d, a0 + off + 2 * j, b0 + off + 2 * j, j > 0, IDESC_F8_M | ncol);
         pre::umma_commit(&done[s]);
         TRACE(3, n);
         s += 2;
@@ -274,7 +260,7 @@ prefill_wide_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
           pre::tc_fence_after();
           const uint64_t off = (uint64_t)(s * (SLOT >> 4));
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_tf32(d, a0 + off + 2 * j, b0 + off + 2 * j, IDESC_TF32_M | ncol, (k > 0 || j > 0) ? 1u : 0u);
+          for (int j = 0; j < 4; ++j) pre::umma_tf32(d, a0 + off + 2 * j, b0 + off + 2 * j, (k > 0 || j > 0) ? 1u : 0u, IDESC_TF32_M | ncol);
           pre::umma_commit(&done[s]);
           if (k == n_z - 1) pre::umma_commit(z_done);
           if (++s == STAGES) { s = 0; ph ^= 1; }

@@ -423,31 +423,31 @@ struct GemmSizes {
 
 // Tiles of 256 tokens (prefill_wide_gemm_kernel) or of 128 (prefill_gemm_kernel)?  Both run one CTA per SM, so a launch
 // takes waves x (K-steps x step + fixed), the steps counted with the residual blocks.  The constants (us) are fitted to
-// the winner of about 2000 launches with each kernel forced on B200 at 1.9 GHz (d_in 128 to 16384, d_out 300 to
-// 40000, 64 to 4096 tokens, 0 / 5 / 15 % residual blocks, residual-only calls, odd and even sizes, both layouts); of 771
-// launches whose waves differ 5 are more than 3 % behind the better kernel, one more than 7 %.  Near the line:
-// 14336 -> 4096, 600 tokens, prepared (1 wave against 2) 109 against 113 us; 14336 -> 28672, 512 tokens, prepared (4
-// against 7) 380 against 355; 4096 -> 6144, 1024 tokens, packed (2 against 3) 83 against 81.
+// the winner of random launches with each kernel forced on B200 at 1.9 GHz (d_in 128 to 28672, d_out 300 to 57344, 64 to
+// 8192 tokens, 0 / 5 / 15 % residual blocks, residual-only calls, odd and even sizes, both layouts).  Of 3865 launches
+// whose waves differ 54 are more than 3 % behind the better kernel; the chosen kernels take 542.9 ms in all, the better
+// ones 541.6.  Near the line: 14336 -> 4096, 600 tokens, prepared (1 wave against 2) 109 against 113 us; 4096 -> 28672, 384 tokens, prepared (4
+// against 5) 101 against 95; 4096 -> 6144, 1024 tokens, packed (2 against 3) 83 against 81.
 // With equally many waves the narrow tile's shorter steps win (14336 -> 4096, 512 tokens, prepared 105 against 64 us),
 // except where mostly the fixed part is left, a few steps of few tokens (512 -> 4096, 128 tokens, packed 10.7 against
 // 11.4; 256 -> 4096, 192 tokens, prepared 8.5 against 9.0).
 // Row-major outputs the narrow kernel stores 64 tokens of a row at a time, with 16-byte stores where these 64 exist and
 // start on 16 bytes and with 2-byte stores scattered over 32 rows where not: every wave of T % 8 != 0 (4096 ->
-// 4096, 2047 tokens, prepared 64 against 141), the last token tile of T % 64 != 0 (640 -> 336, 104 tokens, prepared 10
-// against 14).  The wide kernel stages its stores, so it wins there up to more steps.
+// 4096, 2047 tokens, prepared 64 against 141), the last T % 64 tokens of the others (384 -> 592, 112 tokens, packed 9
+// against 14).  The wide kernel stages its stores, so it wins there up to the more steps the more of them there are.
 bool wants_wide_tiles(const GemmSizes& z, bool prepared, int sm_count) {
   const long long rows = (z.N + 127) / 128;
   const long long w256 = (rows * ((z.T + 255) / 256) + sm_count - 1) / sm_count;
   const long long w128 = (rows * ((z.T + 127) / 128) + sm_count - 1) / sm_count;
   const double n = (z.dense ? z.K / 128 : 0) + (double)z.nnz / (double)rows;
-  const bool scattered = !z.token_major && z.T % 8 != 0, scattered_end = !z.token_major && z.T % 64 != 0;
+  const bool scattered = !z.token_major && z.T % 8 != 0;
   if (w256 == w128) {
     if (scattered) return n <= (prepared ? 60 : 34);
-    if (scattered_end) return n <= (prepared ? 16 : 2.5);
-    return z.token_major && z.dense && ((z.T <= 128 && z.K <= 512) || (prepared && z.T <= 256 && z.K <= 384));
+    if (!z.token_major) return n <= (prepared ? 36 * (z.T % 64) / 64.0 : 18 * (z.T % 64 - 8) / 64.0 + 1) && z.T % 64 != 0;
+    return (z.T <= 128 && z.K <= 512) || (z.T <= 192 && z.K <= 256) || (prepared && (z.K <= 256 || (z.T <= 256 && z.K <= 512)));
   }
-  return prepared ? w256 * (0.74 * n + 2.5) <= w128 * (0.37 * n + (scattered ? 18.0 : 7.0))
-                  : w256 * (1.04 * n + 2.5) <= w128 * (0.55 * n + (scattered ? 16.0 : 4.5));
+  return prepared ? w256 * (0.66 * n + 2.7) <= w128 * (0.37 * n + (scattered ? 20.0 : 6.1))
+                  : w256 * (1.09 * n + 5.7) <= w128 * (0.55 * n + (scattered ? 19.0 : 8.1));
 }
 
 struct GemmChoice {
