@@ -61,7 +61,7 @@ WINDOWS = 3
 NCU_TRAFFIC = {
     ("decode", "packed"): (30.49e6, "decode_gemm_kernel<1|2,false>, mean of the 12 launches", "2026-11-25"),
     ("gate_up_m16", "packed"): (65.82e6, "decode_gemm_kernel<2,false>", "2026-11-25"),
-    ("prefill_gate_up", "prepared"): (226.5e6, "prefill_gemm_kernel<false,true,true>", "2026-11-25"),
+    ("prefill_gate_up", "prepared"): (224.8e6, "prefill_wide_gemm_kernel<true>", "2026-12-03"),
     ("prefill_gate_up", "packed"): (155.0e6, "prefill_gemm_kernel<false,false,false>", "2026-11-25"),
 }
 
@@ -757,6 +757,11 @@ def main():
         achieved = bytes_gemm / gemm_s / 1e9
     value = world * ops_step / (ms_dev / 1e3 / args.steps) / 1e12
     e2e_val = world * ops_step / (ms_e2e / 1e3 / e2e_steps) / 1e12
+    # the GEMM launches on expanded activations: s8 codes on packed weights run the 128-token kernel, prepared weights either
+    names = {_lib.KERNEL_TILES_256: "prefill_wide_gemm_kernel"}
+    gemm_kernels = "decode_gemm_kernel" if not many_tokens else "+".join(sorted({
+        names.get(ops.gemm_choice(it["M"], it["N"], it["K"], it["W"][0].n_hp_blocks, prepared=True, token_major=True)[0] if use_prepared else None,
+                  "prefill_gemm_kernel") for it in data}))
     traffic = NCU_TRAFFIC.get((args.workload, "prepared" if use_prepared else "packed"))
 
     out = {
@@ -784,7 +789,7 @@ def main():
                      "traffic": traffic[0] if traffic else None,
                      "traffic_source": f"{traffic[1]}, captured {traffic[2]}" if traffic else None,
                      "peak_kind": peak_kind,
-                     "kernel": "prefill_gemm_kernel" if many_tokens else "decode_gemm_kernel",
+                     "kernel": gemm_kernels,
                      "us_per_launch": gemm_s / len(data) * 1e6, "bytes_per_launch": bytes_gemm / len(data),
                      "per_shape": per_shape or None},
         "clocks": clk.summary(),

@@ -426,8 +426,9 @@ struct GemmSizes {
 // the winner of random launches with each kernel forced on B200 at 1.9 GHz (d_in 128 to 28672, d_out 300 to 57344, 64 to
 // 8192 tokens, 0 / 5 / 15 % residual blocks, residual-only calls, odd and even sizes, both layouts).  Of 3865 launches
 // whose waves differ 54 are more than 3 % behind the better kernel; the chosen kernels take 542.9 ms in all, the better
-// ones 541.6.  Near the line: 14336 -> 4096, 600 tokens, prepared (1 wave against 2) 109 against 113 us; 4096 -> 28672, 384 tokens, prepared (4
-// against 5) 101 against 95; 4096 -> 6144, 1024 tokens, packed (2 against 3) 83 against 81.
+// ones 541.6.  Near the line (wide against narrow): 14336 -> 4096, 600 tokens, prepared, 1 wave against 2, 109 against
+// 113 us; 4096 -> 28672, 384 tokens, prepared, 4 against 5, 101 against 95; 4096 -> 6144, 1024 tokens, packed, 2
+// against 3, 83 against 81.
 // With equally many waves the narrow tile's shorter steps win (14336 -> 4096, 512 tokens, prepared 105 against 64 us),
 // except where mostly the fixed part is left, a few steps of few tokens (512 -> 4096, 128 tokens, packed 10.7 against
 // 11.4; 256 -> 4096, 192 tokens, prepared 8.5 against 9.0).
