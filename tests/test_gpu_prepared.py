@@ -1,5 +1,5 @@
-"""The many-token kernel's two instantiations - integer MMAs on s8 codes against the packed
-nibbles, and fp8 MMAs (tcgen05 kind::f8f6f4, fp32 accumulation) on weights prepared once as e4m3
+"""The many-token kernels - integer MMAs on s8 codes against the packed nibbles (128-token tiles), fp8 MMAs on nibbles the
+kernel widens to e4m3 (256-token tiles), and fp8 MMAs (tcgen05 kind::f8f6f4, fp32 accumulation) on weights prepared once as e4m3
 bytes - must give the same accumulators and the same output bits: the products and sums are small
 integers, exact in fp32."""
 
@@ -79,7 +79,7 @@ def test_prepared_outputs_equal_packed(ops, T, N, K, density):
     prep = prepare(ops, Wd)
     Xd = X.cuda()
     q = ops.activation_quant_cuda(Xd, Wd.perm)
-    Yp = fused(ops, Wd, q, force="tensor")                       # packed weights, integer MMAs
+    Yp = fused(ops, Wd, q, force="tensor")                       # packed weights, the tile the library picks (128: integer MMAs)
     Yf = fused(ops, Wd, q, force="tensor", prepared=prep)        # prepared weights, fp8 MMAs
     assert torch.equal(Yf, Yp)
     XE8, sumxf8 = ops.expand_activations_cuda(q[0], q[2])        # the same through caller-expanded s8 codes
