@@ -30,7 +30,7 @@ FILES = [
 def install(reference_root: str = "/root/reference") -> bool:
     """Returns True when the files are in place afterwards."""
     dst_root = os.path.join(HERE, "_ref", "kernel")
-    if not os.path.isdir(reference_root):
+    if not all(os.path.isfile(os.path.join(reference_root, f)) for f in FILES):      # no tree, or an empty one
         return all(os.path.exists(os.path.join(dst_root, f)) for f in FILES)
     for rel in FILES:
         src = os.path.join(reference_root, rel)
